@@ -62,3 +62,16 @@ def test_masked_and_unsound_cells_leave_their_neighbours_alone():
     assert np.max(np.abs(v[sound] - want["visc"][sound]) / np.abs(want["visc"][sound])) <= 5e-14
     assert np.max(np.abs(d[sound].T - want["diff"][:, sound]) / np.abs(want["diff"][:, sound])) <= 5e-13
     assert np.isnan(v[10]) and np.isnan(d[10]).all()  # (a NaN temperature is clipped to the fits' range)
+
+
+@pytest.mark.parametrize("mech", ["hydrogen", "grimech30", "dme39"])
+def test_diffusivities_beside_the_viscosity_are_those_of_the_division(mech):
+    """The call for both takes the species viscosities from the reciprocal square root, the call for the
+    diffusivities alone from a division. The corrected quotient is the correctly rounded one unless the exact
+    one lies within 2^-100 of a tie, so the two calls agree bit for bit."""
+    chem = capi.FiniteChem(mech, "fp64")
+    Y, T = cells(chem.nspecies, 20_011, 9)
+    sc = torch.from_numpy(np.vstack([Y, T[None]])).cuda()
+    both, alone = chem.mixture_props(sc, visc=True, diff=True), chem.mixture_props(sc, diff=True)
+    torch.cuda.synchronize()
+    assert torch.equal(both["diff"], alone["diff"])

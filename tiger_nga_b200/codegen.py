@@ -399,14 +399,15 @@ class _Gen:
         o.append(f"      const double num = fma(x, fma(x, fma(x, {_d(om[4])}, {_d(om[3])}), {_d(om[2])}), {_d(om[1])});")
         o.append(f"      const double den = fma(x, fma(x, fma(x, fma(x, {_d(om[9])}, {_d(om[8])}), {_d(om[7])}), "
                  f"{_d(om[6])}), {_d(om[5])});")
-        o.append("      // eta = mucoeff sqrt(T) / Omega(T kOverEps) = a / num, a = mucoeff sqrt(T) den; with the")
-        o.append("      // viscosity's 1/sqrt(eta) = num rsqrt(a num) at hand, eta = (a rsqrt(a num))^2 needs no division")
+        o.append("      // eta = mucoeff sqrt(T) / Omega(T kOverEps) = a / num, a = mucoeff sqrt(T) den. With the viscosity's")
+        o.append("      // 1/sqrt(eta) = num rsqrt(a num) at hand, (a rsqrt(a num))^2 and one Newton step on its residual")
+        o.append("      // a - e num (1/num = a rsqrt(a num)^2) give the division's quotient")
         o.append("      const double ae = q[1] * sq * den;")
         o.append("      double e;")
         o.append("      const double u = yk * q[2];")
         o.append("      if (VISC) {")
-        o.append("        const double ri = rsqrt(ae * num), se = ae * ri;")
-        o.append("        e = se * se;")
+        o.append("        const double ri = rsqrt(ae * num), se = ae * ri, e0 = se * se;")
+        o.append("        e = fma(fma(-e0, num, ae), se * ri, e0);")
         o.append("        su[at] = u, sr[at] = num * ri * q[16];")
         o.append("      } else {")
         o.append("        e = ae / num;")
