@@ -34,6 +34,8 @@ BdfCoef make_coef() {
   return c;
 }
 
+// What a captured graph was made for: the call's arguments, and every buffer of the handle that it holds (they
+// grow, and a graph with the old address must not be launched again).
 struct SubstepKey {
   const double* state;
   int64_t ncells, ld;
@@ -46,6 +48,7 @@ struct SubstepKey {
   int* nst;
   int* nni;
   int* status;
+  const void* scratch[7];
   bool operator==(const SubstepKey& o) const { return std::memcmp(this, &o, sizeof(*this)) == 0; }
 };
 
@@ -296,7 +299,8 @@ int substep_run(tng_chem* h, double* state, int64_t ncells, int64_t ld, const do
   int* nni = cell_nni ? cell_nni : (int*)s->nni.ptr;
   int* sts = cell_status ? cell_status : (int*)s->status.ptr;
   if (list && flags != TNG_DEVICE_PTRS) return set_error(TNG_ERR_ARG, "substep: cell lists need device pointers");
-  SubstepKey key{dstate, ncells, dld, list, nlist, ddts, dt, p, plan.kern, budget, passes, nst, nni, sts};
+  SubstepKey key{dstate, ncells, dld, list, nlist, ddts, dt, p, plan.kern, budget, passes, nst, nni, sts,
+                 {s->counters.ptr, s->queue[0].ptr, s->queue[1].ptr, s->resume.ptr, s->nje.ptr, s->save.ptr, s->factors.ptr}};
   int slot = -1;
   for (int i = 0; i < SolverState::kGraphs; ++i)
     if (s->graph[i] && s->key[i] == key) slot = i;
