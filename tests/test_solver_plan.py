@@ -1,0 +1,76 @@
+"""The rule that picks the implicit solver's launch shape (csrc/solver_plan.h), compiled for the host with a
+stand-in for the occupancy query."""
+import json
+import os
+import shutil
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "tiger_nga_b200", "csrc")
+SMS, SM_BYTES, OPTIN = 148, 233_472, 232_448  # B200: shared memory of an SM and of a block
+
+PROGRAM = r"""
+#include <cstdio>
+#include <cstdlib>
+#include "solver_plan.h"
+using namespace tng;
+int main(int argc, char** argv) {
+  long long v[17];
+  for (int i = 0; i < 17; ++i) v[i] = i + 1 < argc ? std::atoll(argv[i + 1]) : 0;
+  const SolverSizes z{(size_t)v[0], (size_t)v[1], (size_t)v[2], (size_t)v[3], (size_t)v[4], (size_t)v[5]};
+  auto resident = [&](int kernel, int threads, size_t smem) {  // by shared memory and by registers
+    const long long by_smem = v[10] / (long long)(smem + 2048), by_regs = 65536 / (v[11 + kernel] * threads);
+    return (int)(by_smem < by_regs ? by_smem : by_regs);
+  };
+  SolverShape s;
+  if (solver_shape(z, (int)v[6], (int)v[7], v[8], 148, v[9] != 0, resident, &s) < 0) return 1;
+  std::printf("{\"kernel\": %d, \"warps\": %d, \"stages\": %d, \"cold\": %d, \"per_sm\": %d, \"smem\": %zu, \"factors\": %zu}",
+              s.kernel, s.warps, s.stages, s.cold, s.per_sm, s.smem, s.factors);
+}
+"""
+K2, K4, K8, K8X2, POOLED = range(5)
+REGS = (255, 255, 178, 128, 168)  # registers of a thread by kernel
+
+
+@pytest.fixture(scope="module")
+def shape(tmp_path_factory):
+    gxx = shutil.which("g++")
+    if not gxx:
+        pytest.skip("no host compiler")
+    d = tmp_path_factory.mktemp("plan")
+    (d / "plan.cpp").write_text(PROGRAM)
+    subprocess.check_call([gxx, "-std=c++17", "-I", CSRC, str(d / "plan.cpp"), "-o", str(d / "plan")])
+
+    def call(sizes, ncells, warps=0, occupancy=0, scratch=True, regs=REGS):
+        args = [*sizes, warps, occupancy, ncells, int(scratch), SM_BYTES, *regs]
+        return json.loads(subprocess.check_output([str(d / "plan"), *map(str, args)]))
+
+    return call
+
+
+def sizes(ns, hot=30_000, cold=10_000, slots=400, factors=0):
+    """Bytes as the layout gives them, for ns species and a typical set of tables."""
+    nv = ns + 1
+    rs = nv + 1 if nv % 2 == 0 else nv
+    return 8 * (slots + 4 * ns + 300), 8 * (nv * rs + 4 * ns), hot, cold, OPTIN, factors
+
+
+FACTORS = 8 * (32 + 8) * 40  # a warp of the pooled kernel
+
+
+@pytest.mark.parametrize("regs", [168, 80])  # one or two blocks of 12 warps by registers
+def test_factors_cover_every_resident_warp(shape, regs):
+    z = (4_000, 1_500, 10_000, 4_000, OPTIN, FACTORS)
+    s = shape(z, 100_000, regs=REGS[:4] + (regs,))
+    assert s["kernel"] == POOLED and s["warps"] == 12 and s["per_sm"] == (1 if regs == 168 else 2)
+    assert s["factors"] == FACTORS * s["warps"] * s["per_sm"] * SMS
+
+
+def test_lines_between_the_shapes(shape):
+    big, small = sizes(36, factors=FACTORS), sizes(9, hot=6_000, cold=2_000, slots=50)
+    assert [shape(big, n)["kernel"] for n in (1, 8 * SMS, 10 * SMS, 10 * SMS + 1)] == [K8, K8, K8, POOLED]
+    assert [shape(small, n)["kernel"] for n in (1, 8 * SMS, 8 * SMS + 1)] == [K8, K8, K8X2]
+    assert shape(big, 10**6, scratch=False)["kernel"] == K8
+    assert [shape(big, 10**6, warps=w)["kernel"] for w in (2, 4, 8, 12)] == [K2, K4, K8, POOLED]
+    assert shape(small, 10**6, warps=12)["kernel"] == K8

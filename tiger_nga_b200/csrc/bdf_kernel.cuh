@@ -3,6 +3,7 @@
 #pragma once
 #include "kernels.cuh"
 #include "solver.cuh"
+#include "solver_plan.h"
 
 namespace tng {
 
@@ -636,7 +637,6 @@ struct SolverKernels {
 
 // The pooled kernel is for matrices that fill shared memory: rows in both halves of a warp (N > 32), five
 // groups of columns (N <= 40).
-constexpr int kPoolWarps = 12;
 template <class LX>
 constexpr BdfKernelFn pooled_kernel() {
   if constexpr (SvT<LX>::NV > 32 && SvT<LX>::NV <= 40)
@@ -676,13 +676,8 @@ struct SolverPlan {
   size_t smem = 0;
   size_t factors = 0;  // bytes of scratch for the factors (pooled kernel)
 };
-// warps / occupancy as configured (tng_cfg: 0 picks the default of the mechanism's size and the number
-// of cells; scratch: whether the caller has memory for the factors)
+// the rule of solver_plan.h for a mechanism's kernels
 int solver_plan(const MechOps* ops, int mixed, int warps, int occupancy, int64_t ncells, int sm_count, bool scratch,
                 SolverPlan* plan);
-// the range of cell counts that share a plan
-inline int solver_size_class(int64_t ncells, int sm_count) {
-  return ncells <= 8LL * sm_count ? 0 : ncells <= 10LL * sm_count ? 1 : 2;
-}
 
 }  // namespace tng

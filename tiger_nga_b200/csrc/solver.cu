@@ -124,48 +124,22 @@ int solver_plan(const MechOps* ops, int mixed, int warps, int occupancy, int64_t
   int optin = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  const size_t own = sizeof(double) * warp_mem_doubles(L), area = sizeof(double) * stage_mem_doubles(L);
-  const size_t hot = sizeof(double) * hot_smem_doubles(L), cold = sizeof(double) * cold_smem_doubles(L);
-  constexpr size_t kStatic = 1024;  // the staged BDF coefficients and the pool's words
-  SolverPlan p;
-  const int cls = solver_size_class(ncells, sm_count);
-  if (k->pooled && scratch && (warps == kPoolWarps || (warps == 0 && cls == 2))) {
-    // As many matrix areas as fit (a warp holds one for about a third of its time). The line is where
-    // the time for 12 warps crosses that for 8, pooled / 8 warps in ms: GRI 1,201 cells 6.25 / 6.02,
-    // 1,500 6.65 / 7.35, 3,000 10.4 / 11.3, 24,273 58.9 / 65.2; DME 1,201 15.2 / 14.5, 1,500 16.2 /
-    // 16.2, 3,000 23.0 / 24.8, 12,000 69.2 / 77.0. Below it eight warps already hold every cell.
-    const size_t fixed = hot + cold + kPoolWarps * own + kStatic;
-    const int fit = fixed < (size_t)optin ? (int)(((size_t)optin - fixed) / area) : 0;
-    if (fit >= kPoolWarps / 3) {
-      p.kern = k->pooled;
-      p.warps = kPoolWarps;
-      p.stages = std::min(fit, kPoolWarps);
-      p.cold = 1;
-      p.smem = hot + cold + kPoolWarps * own + p.stages * area;
-      p.factors = sizeof(double) * GlobalLu<40>::kDoubles * kPoolWarps * (size_t)sm_count;
-    }
-  }
-  if (!p.kern) {
-    p.warps = (warps == 2 || warps == 4) ? warps : 8;
-    int occ = (p.warps == 8 && occupancy == 2) ? 2 : 1;
-    p.kern = p.warps == 2 ? k->bdf2 : p.warps == 4 ? k->bdf4 : occ == 2 ? k->bdf8_occ2 : k->bdf8;
-    // a small matrix leaves shared memory for 16 warps per SM: worth their 128 registers once there are
-    // cells for them (32,768 hydrogen cells: 14.7 ms, 21.5 ms with 8; 64 registers and 32 warps gain nothing)
-    if (warps == 0 && occupancy == 0 && !k->pooled && cls > 0) occ = 2, p.kern = k->bdf8_occ2;
-    p.stages = p.warps;
-    p.smem = hot + p.warps * (own + area);
-    // the Jacobian's term tables go to shared memory whenever the blocks still fit
-    p.cold = (p.smem + cold + kStatic) * occ <= (size_t)optin ? 1 : 0;
-    if (p.cold) p.smem += cold;
-  }
-  cudaError_t e = ensure_dynamic_smem((const void*)p.kern, p.smem);
-  if (e != cudaSuccess) return cuda_error(e, "solver shared memory");
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.kern, p.warps * 32, p.smem);
-  if (e != cudaSuccess) return cuda_error(e, "solver occupancy");
-  if (per_sm < 1) return set_error(TNG_ERR_CUDA, "solver kernel does not fit on an SM (%zu B shared)", p.smem);
-  p.blocks = per_sm * sm_count;
-  *plan = p;
+  const size_t pooled = k->pooled ? sizeof(double) * GlobalLu<40>::kDoubles : 0;
+  const SolverSizes z{sizeof(double) * warp_mem_doubles(L), sizeof(double) * stage_mem_doubles(L),
+                      sizeof(double) * hot_smem_doubles(L), sizeof(double) * cold_smem_doubles(L), (size_t)optin, pooled};
+  const BdfKernelFn kern[] = {k->bdf2, k->bdf4, k->bdf8, k->bdf8_occ2, k->pooled};
+  cudaError_t e = cudaSuccess;
+  auto resident = [&](int kernel, int threads, size_t smem) {
+    int per_sm = 0;
+    e = ensure_dynamic_smem((const void*)kern[kernel], smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern[kernel], threads, smem);
+    return e == cudaSuccess ? per_sm : -1;
+  };
+  SolverShape s;
+  if (solver_shape(z, warps, occupancy, ncells, sm_count, scratch, resident, &s) < 0)
+    return cuda_error(e, "solver occupancy");
+  if (s.per_sm < 1) return set_error(TNG_ERR_CUDA, "solver kernel does not fit on an SM (%zu B shared)", s.smem);
+  *plan = SolverPlan{kern[s.kernel], s.warps, s.stages, s.cold, s.per_sm * sm_count, s.smem, s.factors};
   return TNG_OK;
 }
 
