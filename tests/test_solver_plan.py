@@ -74,3 +74,13 @@ def test_lines_between_the_shapes(shape):
     assert shape(big, 10**6, scratch=False)["kernel"] == K8
     assert [shape(big, 10**6, warps=w)["kernel"] for w in (2, 4, 8, 12)] == [K2, K4, K8, POOLED]
     assert shape(small, 10**6, warps=12)["kernel"] == K8
+
+
+@pytest.mark.parametrize("ns", [9, 20, 31, 40, 42])
+def test_two_blocks_per_sm_only_where_both_are_resident(shape, ns):
+    s = shape(sizes(ns), 10**6)
+    assert (s["kernel"] == K8X2) == (ns <= 20)  # the others' matrices leave no room for a second block
+    assert s["per_sm"] == (2 if s["kernel"] == K8X2 else 1)
+    # as configured where the caller says so
+    assert shape(sizes(ns), 10**6, warps=8, occupancy=2)["kernel"] == K8X2
+    assert shape(sizes(ns), 10**6, warps=8)["kernel"] == K8

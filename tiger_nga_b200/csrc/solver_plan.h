@@ -52,20 +52,25 @@ int solver_shape(const SolverSizes& z, int warps, int occupancy, int64_t ncells,
       s.smem = z.hot + z.cold + kPoolWarps * z.own + s.stages * z.area;
     }
   }
-  if (s.kernel < 0) {
+  auto own_areas = [&](int occ) {  // the kernels with a matrix area per warp
     s.warps = (warps == 2 || warps == 4) ? warps : 8;
-    int occ = (s.warps == 8 && occupancy == 2) ? 2 : 1;
-    // a small matrix leaves shared memory for 16 warps per SM: worth their 128 registers once there are
-    // cells for them (32,768 hydrogen cells: 14.7 ms, 21.5 ms with 8; 64 registers and 32 warps gain nothing)
-    if (warps == 0 && occupancy == 0 && !z.factors && cls > 0) occ = 2;
     s.kernel = s.warps == 2 ? SOLVER_2 : s.warps == 4 ? SOLVER_4 : occ == 2 ? SOLVER_8X2 : SOLVER_8;
     s.stages = s.warps;
     s.smem = z.hot + s.warps * (z.own + z.area);
     // the Jacobian's term tables go to shared memory whenever the blocks still fit
     s.cold = (s.smem + z.cold + kStatic) * occ <= z.optin ? 1 : 0;
     if (s.cold) s.smem += z.cold;
-  }
+  };
+  // A small matrix leaves shared memory for 16 warps per SM: worth their 128 registers once there are cells
+  // for them (32,768 hydrogen cells: 14.7 ms, 21.5 ms with 8; 64 registers and 32 warps gain nothing). With
+  // one block resident the kernel would spill for nothing: 8 warps with the registers they ask for then.
+  const bool two = s.kernel < 0 && warps == 0 && occupancy == 0 && !z.factors && cls > 0;
+  if (s.kernel < 0) own_areas(two || (warps != 2 && warps != 4 && occupancy == 2) ? 2 : 1);
   s.per_sm = resident(s.kernel, 32 * s.warps, s.smem);
+  if (two && s.per_sm >= 0 && s.per_sm < 2) {
+    own_areas(1);
+    s.per_sm = resident(s.kernel, 32 * s.warps, s.smem);
+  }
   if (s.per_sm < 0) return s.per_sm;
   if (s.kernel == SOLVER_POOLED) s.factors = z.factors * s.warps * (size_t)s.per_sm * sm_count;
   *shape = s;
