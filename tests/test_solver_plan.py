@@ -84,3 +84,9 @@ def test_two_blocks_per_sm_only_where_both_are_resident(shape, ns):
     # as configured where the caller says so
     assert shape(sizes(ns), 10**6, warps=8, occupancy=2)["kernel"] == K8X2
     assert shape(sizes(ns), 10**6, warps=8)["kernel"] == K8
+
+
+def test_configured_occupancy_is_honoured(shape):
+    """A caller that sets the blocks per SM and leaves the warps to the default gets the 8-warp kernels."""
+    for z in (sizes(36, factors=FACTORS), sizes(9, hot=6_000, cold=2_000, slots=50)):
+        assert [shape(z, 10**6, occupancy=o)["kernel"] for o in (1, 2)] == [K8, K8X2]

@@ -36,8 +36,9 @@ int solver_shape(const SolverSizes& z, int warps, int occupancy, int64_t ncells,
                  Resident&& resident, SolverShape* shape) {
   constexpr size_t kStatic = 1024;  // the staged BDF coefficients and the pool's words
   const int cls = solver_size_class(ncells, sm_count);
+  const bool pick = warps == 0 && occupancy == 0;
   SolverShape s;
-  if (z.factors && scratch && (warps == kPoolWarps || (warps == 0 && cls == 2))) {
+  if (z.factors && scratch && (warps == kPoolWarps || (pick && cls == 2))) {
     // As many matrix areas as fit (a warp holds one for about a third of its time). The line is where
     // the time for 12 warps crosses that for 8, pooled / 8 warps in ms: GRI 1,201 cells 6.25 / 6.02,
     // 1,500 6.65 / 7.35, 3,000 10.4 / 11.3, 24,273 58.9 / 65.2; DME 1,201 15.2 / 14.5, 1,500 16.2 /
@@ -64,7 +65,7 @@ int solver_shape(const SolverSizes& z, int warps, int occupancy, int64_t ncells,
   // A small matrix leaves shared memory for 16 warps per SM: worth their 128 registers once there are cells
   // for them (32,768 hydrogen cells: 14.7 ms, 21.5 ms with 8; 64 registers and 32 warps gain nothing). With
   // one block resident the kernel would spill for nothing: 8 warps with the registers they ask for then.
-  const bool two = s.kernel < 0 && warps == 0 && occupancy == 0 && !z.factors && cls > 0;
+  const bool two = s.kernel < 0 && pick && !z.factors && cls > 0;
   if (s.kernel < 0) own_areas(two || (warps != 2 && warps != 4 && occupancy == 2) ? 2 : 1);
   s.per_sm = resident(s.kernel, 32 * s.warps, s.smem);
   if (two && s.per_sm >= 0 && s.per_sm < 2) {
