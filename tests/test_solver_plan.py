@@ -25,8 +25,8 @@ int main(int argc, char** argv) {
   };
   SolverShape s;
   if (solver_shape(z, (int)v[6], (int)v[7], v[8], 148, v[9] != 0, resident, &s) < 0) return 1;
-  std::printf("{\"kernel\": %d, \"warps\": %d, \"stages\": %d, \"cold\": %d, \"per_sm\": %d, \"smem\": %zu, \"factors\": %zu}",
-              s.kernel, s.warps, s.stages, s.cold, s.per_sm, s.smem, s.factors);
+  std::printf("{\"kernel\": %d, \"warps\": %d, \"stages\": %d, \"cold\": %d, \"per_sm\": %d, \"smem\": %zu, \"factors\": %zu, \"from\": %d}",
+              s.kernel, s.warps, s.stages, s.cold, s.per_sm, s.smem, s.factors, s.from);
 }
 """
 K2, K4, K8, K8X2, POOLED = range(5)
@@ -90,3 +90,15 @@ def test_configured_occupancy_is_honoured(shape):
     """A caller that sets the blocks per SM and leaves the warps to the default gets the 8-warp kernels."""
     for z in (sizes(36, factors=FACTORS), sizes(9, hot=6_000, cold=2_000, slots=50)):
         assert [shape(z, 10**6, occupancy=o)["kernel"] for o in (1, 2)] == [K8, K8X2]
+
+
+def test_line_of_the_default_shapes(shape):
+    """Where only the device knows the number of cells both sides of the line are launched: each gets the cells that
+    the rule gives it."""
+    for z in (sizes(36, factors=FACTORS), sizes(9, hot=6_000, cold=2_000, slots=50), sizes(31)):
+        at = shape(z, 10**6)["from"]
+        for n in (1, at - 1, at, 10**5):
+            few = n < at
+            assert shape(z, max(n, 1))["kernel"] == shape(z, 1 if few else 10**6)["kernel"]
+    assert [shape(sizes(36, factors=FACTORS), 10**6, **kw)["from"] for kw in (dict(warps=12), dict(occupancy=2))] == [0, 0]
+    assert shape(sizes(31), 10**6)["from"] == 0  # one block resident: one shape

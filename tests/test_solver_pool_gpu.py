@@ -50,3 +50,45 @@ def test_failed_cells_give_their_matrix_area_back():
         got.append((x, cnt["status"]))
     assert torch.equal(got[0][1], got[1][1]) and torch.equal(got[0][0].nan_to_num(), got[1][0].nan_to_num())
     assert int((got[0][1] == 4).sum()) == 86 and int((got[0][1] == 1).sum()) > 100
+
+
+def solver_kernels_of(call):
+    """Device time in us of the solver's kernels in one call, pooled and not."""
+    from torch.profiler import ProfilerActivity, profile
+
+    call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    k = [(e.name, e.device_time) for e in prof.events() if "k_bdf<" in e.name]
+    return sum(t for n, t in k if ", 12, 1," in n), sum(t for n, t in k if ", 12, 1," not in n)
+
+
+def test_cells_counted_on_the_device_get_the_kernel_for_their_number():
+    """A surrogate's fallback list has the batch's capacity, but few cells: they run on the 8-warp kernel, as a batch of
+    that size does; a list of many runs on the pooled one."""
+    import os
+
+    chem = capi.FiniteChem("grimech30", "fp64")
+    sur = capi.Surrogate(chem, judge_cells=0)
+    sur.load(os.path.join(os.path.dirname(capi.__file__), "models", "grimech30.tngs"))
+    sol, dts = state_batch("grimech30", 8_000, 3, side=0)
+    x0, d = torch.from_numpy(sol).cuda(), torch.from_numpy(dts).cuda()
+    x, stats = torch.empty_like(x0), {}
+
+    def call():
+        x.copy_(x0)
+        stats.update(sur.substep(x, d, P))
+
+    pooled, eight = solver_kernels_of(call)
+    n = stats["cells"] - stats["accepted"]
+    assert 20 < n < 1480 and pooled < 50.0 < 500.0 < eight, (n, pooled, eight)
+    sur.set_gate_tol(1e-9)  # every cell falls back
+    pooled, eight = solver_kernels_of(call)
+    assert stats["accepted"] == 0 and eight < 50.0 < 500.0 < pooled, (pooled, eight)
+    # and the batch of all cells is solved as the list was
+    chem.substep(x0, d, P)
+    torch.cuda.synchronize()
+    assert torch.equal(x, x0)
+    sur.close()

@@ -662,10 +662,18 @@ inline const SolverKernels* solver_kernels_for(const SolverKernels* sets, const 
   return sets + (mixed ? 1 : 0);
 }
 
-static __global__ void k_reset_counters(int* a, int* b) {
+// Before a pass: the queue's head and the count of cells left over to zero. With n_in (a count that only the
+// device knows) the pass is launched with two plans: their counts go to split, all cells to the first when
+// there are fewer than `from`, else to the second, and none to the other.
+static __global__ void k_reset_counters(int* head, int* n_out, const int* n_in, int from, int* split) {
   if (threadIdx.x == 0) {
-    *a = 0;
-    if (b) *b = 0;
+    *head = 0;
+    if (n_out) *n_out = 0;
+    if (n_in) {
+      const int n = *n_in;
+      split[0] = n < from ? n : 0;
+      split[1] = n < from ? 0 : n;
+    }
   }
 }
 
@@ -675,6 +683,7 @@ struct SolverPlan {
   int warps = 0, stages = 0, cold = 0, blocks = 0;
   size_t smem = 0;
   size_t factors = 0;  // bytes of scratch for the factors (pooled kernel)
+  int from = 0;        // fewer cells have another plan (SolverShape::from)
 };
 // the rule of solver_plan.h for a mechanism's kernels
 int solver_plan(const MechOps* ops, int mixed, int warps, int occupancy, int64_t ncells, int sm_count, bool scratch,

@@ -65,7 +65,7 @@ struct SolverState {
   SubstepKey key[kGraphs] = {};
   int next_slot = 0;
   int cfg_warps = -1, cfg_occ = -1, cfg_class = -1;  // the configuration and size that `plan` was made for
-  SolverPlan plan;
+  SolverPlan plan, few;  // few: for cell counts below plan.from (no kernel where there are none)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
@@ -139,7 +139,7 @@ int solver_plan(const MechOps* ops, int mixed, int warps, int occupancy, int64_t
   if (solver_shape(z, warps, occupancy, ncells, sm_count, scratch, resident, &s) < 0)
     return cuda_error(e, "solver occupancy");
   if (s.per_sm < 1) return set_error(TNG_ERR_CUDA, "solver kernel does not fit on an SM (%zu B shared)", s.smem);
-  *plan = SolverPlan{kern[s.kernel], s.warps, s.stages, s.cold, s.per_sm * sm_count, s.smem, s.factors};
+  *plan = SolverPlan{kern[s.kernel], s.warps, s.stages, s.cold, s.per_sm * sm_count, s.smem, s.factors, s.from};
   return TNG_OK;
 }
 
@@ -263,11 +263,15 @@ int substep_run(tng_chem* h, double* state, int64_t ncells, int64_t ld, const do
     if ((rc = solver_plan(h->ops, s->dev.mixed, h->cfg.solver_warps, h->cfg.solver_occupancy, ncells, h->sm_count,
                           true, &s->plan)))
       return rc;
+    s->few = SolverPlan{};
+    if (s->plan.from > 0 && (rc = solver_plan(h->ops, s->dev.mixed, h->cfg.solver_warps, h->cfg.solver_occupancy, 1,
+                                              h->sm_count, true, &s->few)))
+      return rc;
     s->cfg_class = cls;
     s->cfg_warps = h->cfg.solver_warps;
     s->cfg_occ = h->cfg.solver_occupancy;
   }
-  const SolverPlan& plan = s->plan;
+  const SolverPlan &plan = s->plan, &few = s->few;
   if (!s->factors.reserve(plan.factors)) return set_error(TNG_ERR_CUDA, "tng_substep_batch: scratch for the factors");
   int* nst = cell_nst ? cell_nst : (int*)s->nst.ptr;
   int* nni = cell_nni ? cell_nni : (int*)s->nni.ptr;
@@ -310,13 +314,12 @@ int substep_run(tng_chem* h, double* state, int64_t ncells, int64_t ld, const do
     a.status = sts;
     a.smem_warp = warp_mem_doubles(s->dev.L);
     a.smem_stage = stage_mem_doubles(s->dev.L);
-    int* cnt = (int*)s->counters.ptr;  // [0..1] heads, [2..3] out counts
-    L.cold_in_smem = plan.cold;
-    L.stages = plan.stages;
+    int* cnt = (int*)s->counters.ptr;  // [0..1] heads, [2..3] out counts, [4..5] a pass's count by plan
     L.factors = (double*)s->factors.ptr;
     cudaStream_t st = h->stream;
-    if ((e = ensure_dynamic_smem((const void*)plan.kern, plan.smem)) != cudaSuccess)
-      return cuda_error(e, "solver shared memory");
+    for (const SolverPlan* q : {&plan, &few})
+      if (q->kern && (e = ensure_dynamic_smem((const void*)q->kern, q->smem)) != cudaSuccess)
+        return cuda_error(e, "solver shared memory");
     cudaError_t pending = cudaGetLastError();  // an earlier asynchronous error is reported, not captured
     if (pending != cudaSuccess) return cuda_error(pending, "implicit substep (error pending before the graph capture)");
     cudaError_t first = cudaSuccess;            // the first error inside the capture, and where
@@ -324,21 +327,31 @@ int substep_run(tng_chem* h, double* state, int64_t ncells, int64_t ld, const do
     auto note = [&](cudaError_t r, const char* w) {
       if (first == cudaSuccess && r != cudaSuccess) first = r, where = w;
     };
+    auto launch = [&](const SolverPlan& q, const int* n_in) {
+      L.cold_in_smem = q.cold;
+      L.stages = q.stages;
+      L.n_in_dev = n_in;
+      q.kern<<<q.blocks, q.warps * 32, q.smem, st>>>(L);
+      note(cudaGetLastError(), "solver kernel");
+    };
     note(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
     note(cudaMemsetAsync(s->resume.ptr, 0, ncells * sizeof(int), st), "resume flags");
     for (int pass = 0; pass < passes; ++pass) {
       const int cur = pass & 1;
       a.head = cnt + cur;
       a.n_out = cnt + 2 + cur;
-      k_reset_counters<<<1, 32, 0, st>>>(a.head, a.n_out);
+      // The cells of a list, and those that a pass left over, are counted on the device only: both plans are
+      // launched, and the one that the count is not for finds no cells.
+      const int* n_in = pass == 0 ? nlist : cnt + 2 + (cur ^ 1);
+      const bool both = n_in && few.kern;
+      k_reset_counters<<<1, 32, 0, st>>>(a.head, a.n_out, both ? n_in : nullptr, plan.from, cnt + 4);
       note(cudaGetLastError(), "counter reset");
       a.queue_in = pass == 0 ? list : (const int*)s->queue[cur ^ 1].ptr;
       a.queue_out = (int*)s->queue[cur].ptr;
       a.n_in = (int)ncells;
-      L.n_in_dev = pass == 0 ? nlist : cnt + 2 + (cur ^ 1);
       a.budget = pass == passes - 1 ? 0x7fffffff : budget;
-      plan.kern<<<plan.blocks, plan.warps * 32, plan.smem, st>>>(L);
-      note(cudaGetLastError(), "solver kernel");
+      if (both) launch(few, cnt + 4);
+      launch(plan, both ? cnt + 5 : n_in);
     }
     cudaGraph_t graph = nullptr;
     e = cudaStreamEndCapture(st, &graph);

@@ -21,6 +21,7 @@ struct SolverSizes {  // bytes
 struct SolverShape {
   int kernel = -1, warps = 0, stages = 0, cold = 0, per_sm = 0;  // cold: term lists in shared memory
   size_t smem = 0, factors = 0;                                  // factors: of all the grid's warps
+  int from = 0;  // fewer cells than this have another shape by default (0: all have this one)
 };
 
 // the range of cell counts that share a shape
@@ -73,6 +74,8 @@ int solver_shape(const SolverSizes& z, int warps, int occupancy, int64_t ncells,
     s.per_sm = resident(s.kernel, 32 * s.warps, s.smem);
   }
   if (s.per_sm < 0) return s.per_sm;
+  if (pick && s.kernel == SOLVER_POOLED) s.from = 10 * sm_count + 1;
+  if (pick && s.kernel == SOLVER_8X2) s.from = 8 * sm_count + 1;
   if (s.kernel == SOLVER_POOLED) s.factors = z.factors * s.warps * (size_t)s.per_sm * sm_count;
   *shape = s;
   return 0;
