@@ -3,6 +3,8 @@ warp and the 8 of a matrix product, species counts that fill the 8 x 4 fragments
 masked cells, and cells that hold absent, negative or non-finite mass fractions next to sound ones.
 
 Tolerance: sums of at most 40 terms of one sign, a dozen roundings each: 40 * 12 * 2^-53 = 5e-14."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -75,3 +77,46 @@ def test_diffusivities_beside_the_viscosity_are_those_of_the_division(mech):
     both, alone = chem.mixture_props(sc, visc=True, diff=True), chem.mixture_props(sc, diff=True)
     torch.cuda.synchronize()
     assert torch.equal(both["diff"], alone["diff"])
+
+
+def device_transport(chem, sc, visc, diff, mask, nx, ny, nz):
+    """tng_chem_transport on device arrays of a padded block (species at 1..N, T at N+1)."""
+    ns = chem.nspecies
+    e = capi.Extent(imino=1, imaxo=nx, jmino=1, jmaxo=ny, kmino=1, kmaxo=nz, imin=1, imax=nx, jmin=1, jmax=ny, kmin=1,
+                    kmax=nz, nscalar=ns + 1, isc_sc=1, isc_T=ns + 1, isc_H2O=0, isc_CO=0, isc_CO2=0)
+    capi._check(chem.lib.tng_chem_transport(chem.h, visc.data_ptr(), diff.data_ptr(), sc.data_ptr(), mask.data_ptr(),
+                                            ctypes.byref(e), None, 0, capi.TNG_DEVICE_PTRS), "tng_chem_transport")
+
+
+def test_masked_warps_do_no_work():
+    """A block whose masked cells fill whole warps: the others are those of the unmasked call, the masked ones keep
+    their values, and a block that is masked throughout takes the time of reading its mask (a twentieth of the
+    whole block's time or less; the bound leaves a factor of four)."""
+    chem = capi.FiniteChem("grimech30", "fp64")
+    nx, ny, nz = 96, 64, 64
+    n = nx * ny * nz
+    Y, T = cells(chem.nspecies, n, 11)
+    sc = torch.from_numpy(np.vstack([Y, T[None]])).cuda()
+    time = {}
+    for name in ("none", "half", "all"):
+        mask = torch.zeros(ny, nx, dtype=torch.int32, device="cuda")
+        mask[:, 32:] = 1 if name == "all" else 0
+        mask[:, :32] = 0 if name == "none" else 1
+        visc, diff = torch.full((n,), -7.0, device="cuda").double(), torch.full_like(sc, -9.0)
+        torch.cuda.synchronize()
+        for _ in range(3):
+            device_transport(chem, sc, visc, diff, mask, nx, ny, nz)
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        with torch.cuda.stream(chem.torch_stream()):
+            a.record()
+            for _ in range(20):
+                device_transport(chem, sc, visc, diff, mask, nx, ny, nz)
+            b.record()
+        chem.sync()
+        time[name] = a.elapsed_time(b)
+        off = (mask == 1).expand(nz, ny, nx).reshape(-1)
+        if name == "none":
+            want = visc, diff
+        assert bool((visc[off] == -7.0).all()) and bool((diff[:, off] == -9.0).all())
+        assert torch.equal(visc[~off], want[0][~off]) and torch.equal(diff[:, ~off], want[1][:, ~off])
+    assert time["all"] <= 0.2 * time["none"], time

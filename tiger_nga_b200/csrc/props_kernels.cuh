@@ -11,8 +11,9 @@
 // which sets 12 warps per SM for 36 species). Both parts share the FP64 pipe: 8,640 of its cycles per
 // warp in the product (16 per m8n8k4 product), about half as many in the species' fits. GRI, 1,064,895
 // cells, viscosity and diffusivities: 0.998 ms with three scalar FMAs per pair and matrix entry (8
-// warps per SM) -> 0.818 ms -> 0.768 ms with the fits' divisions folded into one rsqrt and the
-// product's steps unrolled; viscosity alone 0.717 -> 0.595 ms (12.0 TFLOP/s counted, 33 % of the pipe).
+// warps per SM) -> 0.818 ms -> 0.77 ms with the fits' divisions folded into one rsqrt (and one Newton step
+// for eta) and the product's steps unrolled; viscosity alone 0.717 -> 0.595 ms (12.0 TFLOP/s counted, 33 %
+// of the pipe).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -117,12 +118,13 @@ __global__ void __launch_bounds__(kPropsBlock) k_props(PropsArgs a) {
       const long long j = (c / a.nxo) % a.nyo;
       live = __ldg(a.mask + i + (long long)a.nxo * j) != 1;
     }
+    const unsigned all = __ballot_sync(0xffffffffu, live);
+    if (!all) continue;  // every cell masked (a wall): no work for the warp
     const double T = live ? __ldcs(a.T + c) : 300.0;
     double lc = 0.0;
     Mech::template transport<LM, VISC, DIFF>(a.y + c, a.ldy, live, T, su, sr, lane, &lc);
     if constexpr (VISC) {
-      const unsigned all = __ballot_sync(0xffffffffu, live);  // (also: every lane's u and rho are stored)
-      __syncwarp();
+      __syncwarp();  // every lane's u and rho are stored
       wilke_visc<Mech, LM>(su, sr, a.visc + base, all, lane);
       __syncwarp();  // u and rho are no longer read
     }
