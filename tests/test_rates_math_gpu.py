@@ -65,3 +65,24 @@ def test_arguments_outside_the_exponentials_range(mech):
         assert not np.isfinite(a[over]).any()
         assert np.isfinite(a[~over & ~np.isnan(b)]).all()
         assert np.isnan(W[i, -1])
+
+
+@pytest.mark.parametrize("mech", ["hydrogen", "grimech30", "dme39"])
+def test_arguments_stay_in_range_at_any_temperature(mech):
+    """Temperatures of states that have gone wrong (a density near zero, an infinity): the exponentials' arguments
+    are held in the tables' range, so a rate that is finite comes out as the oracle's, one that vanishes vanishes
+    and one that overflows is not finite."""
+    m = load(mech)
+    T = np.concatenate([10.0 ** np.linspace(8.0, 14.0, 1500), [0.0, np.inf]])
+    sol = cells(m.ns, T, 1.0, 10)
+    W, Wo = slot_rates(mech, sol)
+    emax = max(abs(a.E) for s in m.slots for a in ((s.k0, s.kinf) if s.kind == "falloff" else (s.arr,)) if a.E is not None)
+    for i, s in enumerate(m.slots):
+        a, b = W[i], Wo[i]
+        finite = np.isfinite(b) & np.isfinite(T) & (np.abs(b) > 1e-280) & (T > 0.0)
+        # |ln W| < 645, n ln T below 600: the roundings of sums up to 1,400 on either side
+        assert (np.abs(a[finite] - b[finite]) <= 2e-12 * np.abs(b[finite])).all(), s.index
+        if s.kind == "falloff" or abs(s.arr.n or 0.0) < 0.1 or abs(s.arr.E or 0.0) < 1e-3 * emax:
+            continue  # small exponents need not have saturated at the bounds
+        assert (np.abs(a[b == 0.0]) <= 1e-290).all(), s.index
+        assert not np.isfinite(a[np.isinf(b)]).any(), s.index

@@ -72,9 +72,13 @@ class _Gen:
         self.m64 = Mechanism(name, "f64")
         m = self.m32
         self.ns, self.nslot, self.nm = m.ns, m.nslot, m.nm
-        # largest |activation energy|: bounds the arguments of the table exponential
+        # what bounds the arguments of the table exponential: the largest |activation energy| and temperature
+        # exponent, the smallest scale of a T / x in F_cent that takes it
         arr = [a for s in m.slots for a in ((s.k0, s.kinf) if s.kind == "falloff" else (s.arr,))]
         self.emax = max([abs(a.E) for a in arr if a.E is not None] + [1.0])
+        self.nmax = max([abs(a.n) for a in arr if a.n is not None] + [1.0])
+        fc = [t for s in m.slots if s.kind == "falloff" for t in s.fc_key]
+        self.xmin = min([x for _, form, x in fc if form == 0 and x >= 1.0] + [1e20])
         # first slot that needs each third-body set (as W factor or as falloff [M])
         self.fc_keys32: dict[tuple, int] = {}
 
@@ -95,7 +99,7 @@ class _Gen:
 
     def fc_code(self, idx: int, fc32, fc64, out: list[str], prec: str):
         """Emit F_cent for one distinct expression; returns the names of log10(fc), log2(fc)."""
-        terms = []
+        terms, hot = [], []
         for (a, form, x), (a6, _, x6) in zip(fc32, fc64):
             # exact shortcuts: exp(-T/1e30) == 1.0 and exp(-T/1e-30) == 0.0 in double for any T in range
             if form == 0 and x <= 1e-20:
@@ -105,10 +109,15 @@ class _Gen:
             if (form == 0 and x >= 1e20) or (form == 1 and x == 0.0):
                 terms.append(_lm(a, a6))
                 continue
-            # the table exponential needs |argument| < 5e6: T / x with x >= 1, x / T with T at its bound
-            table = prec == "fp64" and (x >= 1.0 if form == 0 else x * self.m32.rgas <= self.emax)
+            # the table exponential needs |argument| < 5e6: x / T from T at its bound; T / x is given up (to
+            # zero) from T = 4e6 of the smallest x on, by a selection (a bounded copy of T would be two more
+            # registers: 3,024 bytes of spilled loads for GRI, 2,296 so)
+            table = prec == "fp64" and (x >= 1.0 if form == 0 else abs(x) * self.m32.rgas <= self.emax)
             e = f"-T * {_lm(1.0 / x, 1.0 / x6)}" if form == 0 else f"-{_lm(x, x6)} * invT{'e' if table else ''}"
-            terms.append(f"{_lm(a, a6)} * " + (f"tng_exp({e}, xt)" if table else f"exp({e})"))
+            term = f"{_lm(a, a6)} * " + (f"tng_exp({e}, xt)" if table else f"exp({e})")
+            (hot if table and form == 0 else terms).append(term)
+        if hot:
+            terms.insert(0, f"(T > {_d(4e6 * self.xmin)} ? 0.0 : {' + '.join(hot)})")
         if not terms:
             raise ValueError("F_cent is identically zero")
         out.append(f"  const double fc{idx} = {' + '.join(terms)};")
@@ -144,10 +153,12 @@ class _Gen:
         o.append("  const double LT = log(T);")
         o.append(f"  const double invRT = 1.0 / ({_lm(m32.rgas, m64.rgas)} * T);")
         o.append(f"  const double invT = {_lm(m32.rgas, m64.rgas)} * invRT;")
-        # The table exponentials need |E/(R T)| < 2e6: a bound on T of a few hundredths of a kelvin, where
-        # they are zero or infinite but for the smallest E; below it the argument stays (as does a NaN).
-        for v, scale in (("invRT", 1.0), ("invT", m64.rgas)) if prec == "fp64" else ():
-            b = _d(2e6 / self.emax * scale)
+        # The table exponentials need |argument| < 5e6, which these bounds give: |E/(R T)| <= 2e6 (T above a few
+        # hundredths of a kelvin), |n ln T| <= 4e5 (any T but zero and infinity). Past a bound the argument stays,
+        # where the exponential is zero or infinite but for the smallest E and n. A NaN passes.
+        bounds = [("invRT", 2e6 / self.emax), ("invT", 2e6 / self.emax * m64.rgas), ("LT", 4e5 / self.nmax)]
+        for v, bound in bounds if prec == "fp64" else ():
+            b = _d(bound)
             o.append(f"  const double {v}e = {v} > {b} ? {b} : {v} < -{b} ? -{b} : {v};")
         for k in range(ns):
             o.append(f"  const double c{k} = s[{k}] * {_lm(1.0 / m32.wmol[k], 1.0 / m64.wmol[k])};")
@@ -210,14 +221,14 @@ class _Gen:
                 lnA0, n0, E0 = self.arr_terms(s32.k0, s64.k0, False)
                 lnAi, ni, Ei = self.arr_terms(s32.kinf, s64.kinf, False)
 
-                invRT = "invRTe" if prec == "fp64" else "invRT"
+                invRT, LT = ("invRTe", "LTe") if prec == "fp64" else ("invRT", "LT")
 
                 def expo(lnA, n, E):
                     e = lnA
                     if E is not None:
                         e = f"fma({E}, {invRT}, {e})"
                     if n is not None:
-                        e = f"fma({n}, LT, {e})"
+                        e = f"fma({n}, {LT}, {e})"
                     return e
 
                 kmin = math.log(m32.troe["kmin"])
@@ -274,7 +285,7 @@ class _Gen:
                     if E is not None:
                         e = f"fma({E}, invRTe, {e})"
                     if n is not None:
-                        e = f"fma({n}, LT, {e})"
+                        e = f"fma({n}, LTe, {e})"
                     o.append(f"  {{ double w = tng_exp({e}, xt);")
                 for c in s32.C:
                     o.append(f"    w = w * c{c};")
