@@ -207,7 +207,11 @@ __device__ __forceinline__ void constraint_col(const SurPost& a, const PostTab& 
 // projection repeated over the rest (an active set), so clipping keeps the constraints. A
 // constraint whose carriers are all pinned or absent (G_ee = 0) holds already when its residual
 // is zero and is then left out; otherwise, or when the active set does not settle, the cell is
-// rejected (returns false).
+// rejected (returns false). So it is when the constraints are nearly dependent on the species that are
+// left, a pivot being below kMinPivot of its diagonal: the solve is off by about 2^-53 over the pivot, 1e-8 of
+// an element's mass at the limit (1e-2 at 1e-14, where the factorisation itself would still go through). None
+// of 523,777 GRI cells has a pivot below 1e-5.
+constexpr double kMinPivot = 1e-8;
 template <int NC, int NEL>
 __device__ __forceinline__ bool project(const SurPost& a, const PostTab& t, const CellY& Y0, double* dY, float* D,
                                         double Th, double hsc, double hrhs) {
@@ -259,7 +263,7 @@ __device__ __forceinline__ bool project(const SurPost& a, const PostTab& t, cons
 #pragma unroll
         for (int q = 0; q < j; ++q) sg -= G[i][q] * G[j][q];
         if (i == j) {
-          if (!(sg > 1e-14 * G[i][i])) return false;  // dependent constraints
+          if (!(sg > kMinPivot * G[i][i])) return false;  // dependent constraints
           G[i][i] = sqrt(sg);
         } else {
           G[i][j] = sg / G[j][j];
