@@ -171,7 +171,8 @@ typedef struct tng_substep_stats {
  * work-stealing kernel; the pass loop runs as one CUDA graph. cell_nst / cell_nni / cell_status
  * (device int arrays of ncells, nullable) receive per-cell step and Newton counts and status
  * (0 ok, 1 max steps, 2 convergence failures, 3 error-test failures, 4 non-finite, 5 step too
- * small). flags: TNG_DEVICE_PTRS (state, dts and cell arrays on the device) or TNG_HOST_PTRS
+ * small, 6 no memory for a factorisation: not unless the solver itself is at fault).
+ * flags: TNG_DEVICE_PTRS (state, dts and cell arrays on the device) or TNG_HOST_PTRS
  * (state and dts on the host; cell arrays must then be null). stats may be null; when given the
  * call waits for the device. */
 int tng_substep_batch(tng_chem* h, double* state, int64_t ncells, int64_t ld, const double* dts, double dt, double p,

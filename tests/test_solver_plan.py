@@ -2,6 +2,7 @@
 stand-in for the occupancy query."""
 import json
 import os
+import re
 import shutil
 import subprocess
 
@@ -102,3 +103,24 @@ def test_line_of_the_default_shapes(shape):
             assert shape(z, max(n, 1))["kernel"] == shape(z, 1 if few else 10**6)["kernel"]
     assert [shape(sizes(36, factors=FACTORS), 10**6, **kw)["from"] for kw in (dict(warps=12), dict(occupancy=2))] == [0, 0]
     assert shape(sizes(31), 10**6)["from"] == 0  # one block resident: one shape
+
+
+def test_every_status_is_documented_and_leaves_an_accepted_state():
+    """The statuses of the kernel are those the public header lists, and an exit between a step's prediction and
+    its acceptance takes the prediction back first (the cell's state is written as it then is)."""
+    def read(*p):
+        with open(os.path.join(CSRC, *p)) as f:
+            return f.read()
+
+    enum = re.search(r"enum \{ (ST_OK[^}]*)\}", read("solver.cuh")).group(1)
+    codes = {int(v): k for k, v in re.findall(r"(ST_\w+) = (\d+)", enum) if k != "ST_PENDING"}
+    doc = " ".join(read("..", "..", "include", "tiger_chem.h").replace("\n *", " ").split())
+    listed = re.search(r"status \((0 ok, .*?)\)", doc).group(1)
+    assert [int(v) for v in re.findall(r"(?:^|, )(\d) ", listed)] == sorted(codes)
+    kernel = read("bdf_kernel.cuh")
+    attempt = kernel[kernel.index("z_predict<two>(z, q);"):kernel.index("// accept\n")]
+    failing = [m.start() for m in re.finditer(r"\bfail = true;", attempt)]
+    assert failing
+    for at in failing:
+        block = attempt[attempt.rindex("if (uni(", 0, at) - 250:at]
+        assert "z_retract<two>(z, q);" in block, block

@@ -311,6 +311,7 @@ __device__ __forceinline__ bool bdf_cell(const BdfLaunch& P, const BdfCoef& C, c
           if constexpr (POOL) {
             area = pool_take(pool, lane);
             if (uni(area < 0)) {
+              z_retract<two>(z, q);
               status = ST_NOAREA;
               fail = true;
               break;
