@@ -798,13 +798,9 @@ class Mlp:
         return losses
 
     def _sync_in(self):
-        import torch
-
         self.chem._fork(self.chem.device)
 
     def _sync_out(self):
-        import torch
-
         self.chem._join(self.chem.device)
 
 
@@ -848,13 +844,9 @@ class Surrogate:
             pass
 
     def _pre(self):
-        import torch
-
         self.chem._fork(self.chem.device)
 
     def _post(self):
-        import torch
-
         self.chem._join(self.chem.device)
 
     def train(self, state0, state1, dts, p: float, epochs: int = 10, batch: int = 4096, lr: float = 1e-3):

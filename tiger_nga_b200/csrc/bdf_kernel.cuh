@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) k_bdf(const BdfLaunch P) {
   double* wb = smem + off + (size_t)warp * P.a.smem_warp;
   double* areas = smem + off + (size_t)WARPS * P.a.smem_warp;
   MatPool pool{&s_free, areas, P.a.smem_stage, nullptr};
-  if constexpr (POOL) pool.fac = P.factors + (size_t)(blockIdx.x * WARPS + warp) * GlobalLu<SvT<LY>::NV>::kDoubles;
+  if constexpr (POOL) pool.fac = P.factors + (size_t)(blockIdx.x * WARPS + warp) * GlobalLu::kDoubles;
   const int n_in = P.n_in_dev ? *P.n_in_dev : P.a.n_in;
   // Few cells are dealt out, block by block before warp by warp, so that they spread over all SMs
   // (claimed from the counter, the blocks that start first would take one per warp).

@@ -124,7 +124,7 @@ int solver_plan(const MechOps* ops, int mixed, int warps, int occupancy, int64_t
   int optin = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  const size_t pooled = k->pooled ? sizeof(double) * GlobalLu<40>::kDoubles : 0;
+  const size_t pooled = k->pooled ? sizeof(double) * GlobalLu::kDoubles : 0;
   const SolverSizes z{sizeof(double) * warp_mem_doubles(L), sizeof(double) * stage_mem_doubles(L),
                       sizeof(double) * hot_smem_doubles(L), sizeof(double) * cold_smem_doubles(L), (size_t)optin, pooled};
   const BdfKernelFn kern[] = {k->bdf2, k->bdf4, k->bdf8, k->bdf8_occ2, k->pooled};

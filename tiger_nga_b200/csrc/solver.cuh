@@ -887,7 +887,6 @@ __device__ __forceinline__ void lu_solve_reg(const double* a, const int n, const
 // shared memory. Column k of rows 0..31 is lo[32 k + lane], of the rows from 32 on hi[8 k + lane]: a lane
 // writes and reads its own rows only. (Tensor memory would hold them nearer, but a kernel with any
 // tcgen05 instruction gets the guarded form of every shuffle, see uni().)
-template <int N>
 struct GlobalLu {
   static constexpr int kGroups = 5;  // groups of eight columns, N <= 40
   static constexpr int kHi = 32 * 8 * kGroups;
@@ -897,7 +896,7 @@ struct GlobalLu {
 // The factors of an N x N LU in shared memory (row stride RS) into the warp's scratch.
 template <int N, int RS>
 __device__ __forceinline__ void lu_to_global(const double* __restrict__ a, double* __restrict__ fac, const int lane) {
-  using L = GlobalLu<N>;
+  using L = GlobalLu;
 #pragma unroll 4
   for (int k = 0; k < N; ++k) {
     fac[32 * k + lane] = a[lane * RS + k];
@@ -910,7 +909,7 @@ __device__ __forceinline__ void lu_to_global(const double* __restrict__ a, doubl
 template <int N>
 __device__ __forceinline__ void lu_solve_global(const double* fac, const int* perm, const double* dinv, double* vb,
                                                 double& x0, double& x1, const int lane) {
-  using L = GlobalLu<N>;
+  using L = GlobalLu;
   static_assert(N > 32 && N <= 40, "rows lane and lane + 32, five groups of columns");
   const bool h1 = lane + 32 < N;
   struct Cols {
