@@ -738,7 +738,7 @@ def main():
                               "frac": fp64_ach / fp64_peak, "alg_flops_per_cell": work_c["flops"],
                               "transcendentals_per_cell": work_c["transcendentals"],
                               "note": "reference-formulation flops (transcendentals counted separately); the "
-                                      "kernel is FP64-pipe bound, the HBM figure is reported per schema"}}
+                                      "kernel is bound by its instructions, the HBM figure is reported per schema"}}
     else:
         # dominant kernel: the implicit solver (k_bdf) -- the whole substep, or the fallback cells
         sst = stats_last if wl["kind"] == "substep" else stats_last["fallback"]

@@ -191,8 +191,8 @@ class _Gen:
 
         if prec == "mixed":
             # All third-body sums first: after them only the logarithms of the concentrations are needed, two
-            # registers fewer per species in a kernel that spills (1,048,576 cells: DME 0.728 -> 0.675 ms, GRI
-            # 1.010 -> 0.987 ms; spilled loads 2,344 -> 1,476 bytes)
+            # registers fewer per species in a kernel that spills (DME: spilled loads 2,344 -> 1,476 bytes; 716,539
+            # cells 0.510 -> 0.493 ms, 1,048,576 0.762 -> 0.707; 2,097,152 GRI cells 2.135 -> 2.062)
             for s32 in m32.slots:
                 for j in ((s32.M_fall,) if s32.kind == "falloff" else ()) + ((s32.M,) if s32.M >= 0 else ()):
                     need_m(j)
